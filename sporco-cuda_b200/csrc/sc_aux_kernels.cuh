@@ -24,18 +24,33 @@ __global__ void psum_kernel(const float2* __restrict__ Dh, float* __restrict__ P
 
 // Psum without the filters' column spectra: |Df_m(kr)|^2 = sum_s R_m(s) w^(s kr)
 // over the lags s of the column autocorrelation R_m(s) = sum_t e_m(t + s)
-// conj(e_m(t)) of the filter rows' spectra e (E, (M, Kr, Wp)), R_m(-s) =
-// conj(R_m(s)); all sums in double precision.  The lags are summed over the maps
-// [m0, M) (R: (Kr, Wp); one CTA per 32 columns and lag, eight map lanes) ...
-__global__ void autocorr_kernel(const float2* __restrict__ E, double2* __restrict__ R, int m0,
-                                int M, int Kr, int Wf, int Wp) {
+// conj(e_m(t)) of the filter rows' spectra e, R_m(-s) = conj(R_m(s)); all sums in
+// double precision.  The lags are summed over the maps [1, M) and, in the second
+// z slice, over map 0; with one slice over all maps (R: (slices, Kr, Wp); one CTA
+// per 32 columns and lag, eight map lanes) ...
+// PAIRS: e as filter_rows_kernel's column pairs, E rows per map; else (M, E, Wp).
+// held: nothing to do if *held has HELD_SPLIT (or NULL).
+template <bool PAIRS>
+__global__ void autocorr_kernel(const float* __restrict__ e, double2* __restrict__ R, int M,
+                                int Kr, int E, int Wf, int Wp, const int* held) {
   __shared__ double2 part[8][32];
+  if (held && (*held & HELD_SPLIT)) return;
   const int c = blockIdx.x * 32 + threadIdx.x, s = blockIdx.y;
+  const int m0 = gridDim.z == 2 && blockIdx.z == 0 ? 1 : 0, m1 = blockIdx.z == 1 ? 1 : M;
+  R += (size_t)blockIdx.z * Kr * Wp;
+  auto at = [&](int m, int t) -> float2 {
+    const size_t r = ((size_t)m * E + t) * Wp;
+    if constexpr (PAIRS) {
+      const float* p = e + (r + (c & ~1)) * 4 + (c & 1);
+      return make_float2(p[0], p[6]);
+    } else {
+      return reinterpret_cast<const float2*>(e)[r + c];
+    }
+  };
   double2 v = make_double2(0.0, 0.0);
-  for (int m = m0 + threadIdx.y; m < M && c < Wf; m += 8) {
-    const float2* e = E + (size_t)m * Kr * Wp + c;
+  for (int m = m0 + threadIdx.y; m < m1 && c < Wf; m += 8) {
     for (int t = 0; t + s < Kr; ++t) {
-      const float2 a = e[(size_t)(t + s) * Wp], b = e[(size_t)t * Wp];
+      const float2 a = at(m, t + s), b = at(m, t);
       v.x += (double)a.x * b.x + (double)a.y * b.y;
       v.y += (double)a.y * b.x - (double)a.x * b.y;
     }
@@ -50,25 +65,38 @@ __global__ void autocorr_kernel(const float2* __restrict__ E, double2* __restric
     R[(size_t)s * Wp + c] = v;
   }
 }
-// ... and summed over the lags: Psum(kr) = R(0) + 2 sum_s Re(R(s) w^(s kr)).
+// ... and summed over the lags: Psum(kr) = R(0) + 2 sum_s Re(R(s) w^(s kr)); with
+// two slices of R also Psum1 of the maps [1, M) and Psum0 of map 0.
 // (Instead of the zero-padded filters' 2-D spectra and a sum over the maps:
 // 2048 x 2048, 256 filters of 16 x 16 11.4 -> 0.3 ms of a solve's set-up, 256 x
 // 256, 64 of 11 x 11 80 -> 20 us.)
-__global__ void psum_lags_kernel(const double2* __restrict__ R, float* __restrict__ Psum, int H,
-                                 int Wf, int Wp, int Kr) {
+__global__ void psum_lags_kernel(const double2* __restrict__ R, float* __restrict__ Psum,
+                                 float* __restrict__ Psum1, float* __restrict__ Psum0, int H,
+                                 int Wf, int Wp, int Kr, const int* held) {
+  if (held && (*held & HELD_SPLIT)) return;
   const int c = blockIdx.x * blockDim.x + threadIdx.x, kr = blockIdx.y;
   if (c >= Wf) return;
-  const double2* r = R + c;
-  double s, w, v = r[0].x;
+  const double2 *r = R + c, *r0 = r + (size_t)Kr * Wp;
+  const bool two = Psum0 != nullptr;
+  double s, w, v = r[0].x, v0 = two ? r0[0].x : 0.0;
   sincospi(-2.0 * (double)kr / (double)H, &s, &w);
   const double2 w1 = make_double2(w, s);
   double2 p = w1;
   for (int k = 1; k < Kr; ++k) {
     const double2 l = r[(size_t)k * Wp];
     v += 2.0 * (l.x * p.x - l.y * p.y);
+    if (two) {
+      const double2 l0 = r0[(size_t)k * Wp];
+      v0 += 2.0 * (l0.x * p.x - l0.y * p.y);
+    }
     p = make_double2(p.x * w1.x - p.y * w1.y, p.x * w1.y + p.y * w1.x);
   }
-  Psum[(size_t)kr * Wp + c] = (float)fmax(v, 0.0);
+  const size_t i = (size_t)kr * Wp + c;
+  Psum[i] = (float)fmax(v + v0, 0.0);
+  if (two) {
+    Psum1[i] = (float)fmax(v, 0.0);
+    Psum0[i] = (float)fmax(v0, 0.0);
+  }
 }
 
 // ============================================================== finalize ==
@@ -146,9 +174,19 @@ __global__ void finalize_kernel(const double* __restrict__ partials, int nblk,
   }
 }
 
-__global__ void init_state_kernel(ImgState* st, const float* rho0, int B, int* ndone) {
+// made: what this call's set-up made of the dictionary (HELD_*); over: in the
+// place of what the workspace held, else in addition to it.
+__device__ __forceinline__ void note_held(int* held, int made, int over) {
+  *held = over ? made : *held | made;
+}
+
+__global__ void init_state_kernel(ImgState* st, const float* rho0, int B, int* ndone, int* held,
+                                  int made, int over) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b == 0 && ndone) *ndone = 0;
+  if (b == 0) {
+    *ndone = 0;
+    note_held(held, made, over);
+  }
   if (b >= B) return;
   ImgState s;
   s.rho = (double)rho0[b];
@@ -167,9 +205,12 @@ __global__ void init_state_kernel(ImgState* st, const float* rho0, int B, int* n
 // A warm-started solve call continues the state of the previous one: rho,
 // the iterates and the iteration count carry over; the call's own cap counts
 // from the current count, and the finished flags start afresh.
-__global__ void warm_state_kernel(ImgState* st, int B, int* ndone) {
+__global__ void warm_state_kernel(ImgState* st, int B, int* ndone, int* held, int made, int over) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b == 0 && ndone) *ndone = 0;
+  if (b == 0) {
+    *ndone = 0;
+    note_held(held, made, over);
+  }
   if (b >= B) return;
   st[b].k0 = st[b].k;
   st[b].done = 0;

@@ -81,6 +81,12 @@ struct ImgState {
   int k0;        // k at the start of the current solve call (its cap counts from here)
 };
 
+// What the workspace holds of the dictionary besides what every set-up leaves
+// there (a flag word on the device; a solve that reuses the spectra, warm_start
+// 2, makes what it needs and an earlier one did not): its 2-D spectrum, and
+// Psum of map 0 and of the others apart.
+enum { HELD_DICT = 1, HELD_SPLIT = 2 };
+
 // Scalar options the finalize kernel needs.
 struct FinParams {
   int max_iter;
@@ -133,6 +139,7 @@ struct RowParams {
   const float* src;        // real rows (B, M, H, W) for ROW_FWD_REAL
   const float* D;          // (M, Kr, Kc) for ROW_FWD_DICT
   int Kr, Kc;
+  const int* held;         // ROW_FWD_DICT: nothing to do if *held has HELD_DICT (or NULL)
   float* dst;              // real rows out for ROW_INV_REAL
   // adjoint (ROW_ADJ)
   float* gV;               // (B, M, H, W) gradient w.r.t. V of the step, in place
@@ -167,6 +174,7 @@ struct ColParams {
   int two;                 // CONV_GRAD: the gradient weight of map 0 is zero
   const double2* twHd;     // column twiddles in double precision (COL_CONV, any length)
   const float* Psum0;      // (H, Wp) |Df_0|^2 (two; Psum is then over the other maps)
+  const int* held;         // COL_FWD: nothing to do if *held has HELD_DICT (or NULL)
   ImgState* st;
   float2* Xtr;             // COL_SOLVE_X: x^ also written here (B, M, H, Wp); COL_SOLVE_C*T:
                            // the row spectra of X (or NULL)

@@ -675,6 +675,9 @@ row_kernel(RowParams P) {
     return;
   } else {
     // ---------------------------------------------- setup and tool modes
+    if constexpr (MODE == ROW_FWD_DICT) {
+      if (P.held && (*P.held & HELD_DICT)) return;
+    }
     for (long pb = (long)blockIdx.x * S; pb < npairs; pb += pstride) {
       const long p = pb + s;
       const bool valid = p < npairs;
@@ -791,6 +794,7 @@ col_kernel(ColParams P) {
   if constexpr (MODE == COL_FWD || MODE == COL_INV) {
     // setup / tool: plain loads (the spectrum pitch may be unaligned here)
     const bool inv = MODE == COL_INV;
+    if (P.held && (*P.held & HELD_DICT)) return;
     for (int m = m0; m < m1; ++m) {
       float2* src = Fi + (size_t)m * H * Wp + c0;
       for (int e = tid; e < T * H; e += NT) {

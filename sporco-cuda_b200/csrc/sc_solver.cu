@@ -147,8 +147,8 @@ struct Plan {
   int colg_g, colg_NT;
   size_t colg_smem, colt_smem;
   int max_iter;
-  size_t off_U, off_F, off_Dh, off_Sh, off_Ps, off_Ps0, off_E, off_twW, off_twH, off_twHd, off_lags, off_part, off_st,
-      off_it, off_xi, off_ndone, off_objspec, off_objpart, total;
+  size_t off_U, off_F, off_Dh, off_Sh, off_Ps, off_Ps0, off_Ps1, off_E, off_twW, off_twH, off_twHd, off_lags, off_part, off_st,
+      off_held, off_it, off_xi, off_ndone, off_objspec, off_objpart, total;
 };
 
 // Process-wide caches of this file (kernel attributes, occupancy answers,
@@ -244,13 +244,15 @@ static int plan_problem(const sc_problem* p, const sc_options* o, Plan* pl) {
   pl->off_Sh = take(sizeof(float2) * (size_t)g.H * g.Wp * g.B);
   pl->off_Ps = take(sizeof(float) * (size_t)g.H * g.Wp);
   pl->off_Ps0 = take(sizeof(float) * (size_t)g.H * g.Wp);
+  pl->off_Ps1 = take(sizeof(float) * (size_t)g.H * g.Wp);
   pl->off_E = take(sizeof(float4) * (size_t)g.M * (p->Kr <= 16 ? conv_pad_taps(p->Kr) : 0) * g.Wp);
   pl->off_twW = take(sizeof(float2) * g.W);
   pl->off_twH = take(sizeof(float2) * g.H);
   pl->off_twHd = take(sizeof(double2) * g.H);
-  pl->off_lags = take(p->Kr <= 16 ? sizeof(double2) * (size_t)p->Kr * g.Wp : 0);
+  pl->off_lags = take(p->Kr <= 16 ? 2 * sizeof(double2) * (size_t)p->Kr * g.Wp : 0);
   pl->off_part = take(sizeof(double) * 5 * (size_t)pl->row_nblk * g.B);
   pl->off_st = take(sizeof(ImgState) * g.B);
+  pl->off_held = take(sizeof(int));
   pl->off_it = take(o->record_itstat ? sizeof(double) * SC_ITSTAT_FIELDS *
                                           (size_t)std::max(1, o->max_iter) * g.B
                                     : 0);
@@ -774,18 +776,23 @@ struct Solve {
     const bool two_d = col_mode == COL_CONV && two;
     float* Erows = (float*)((unsigned char*)workspace + pl.off_E);
     float* Psum0 = (float*)((unsigned char*)workspace + pl.off_Ps0);
+    float* Psum1 = (float*)((unsigned char*)workspace + pl.off_Ps1);
+    int* held = (int*)((unsigned char*)workspace + pl.off_held);
     const int Ep = p->Kr <= 16 ? conv_pad_taps(p->Kr) : 0;
 
-    // warm_start 2: the spectra of D and S in the workspace are still valid
+    // warm_start 2: the spectra of D and S in the workspace are still valid.
+    // What every set-up leaves there serves any later call; what only some
+    // make (HELD_*) a call that needs it makes then, if it is not there.
     const bool spectra = o->warm_start != 2;
+    const bool twd = conv && !spec_col(g.H);
     if (spectra) {
       twiddle_kernel<<<(g.W + 255) / 256, 256, 0, s>>>(twW, g.W);
       twiddle_kernel<<<(g.H + 255) / 256, 256, 0, s>>>(twH, g.H);
-      if (col_mode == COL_CONV && !spec_col(g.H))
+      if (twd)
         twiddle_d_kernel<<<(g.H + 255) / 256, 256, 0, s>>>(
             (double2*)((unsigned char*)workspace + pl.off_twHd), g.H);
       CU_TRY(cudaGetLastError());
-      g_launches += 2 + (col_mode == COL_CONV && !spec_col(g.H));
+      g_launches += 2 + twd;
     }
 
     // Dictionary.  The convolution column pass takes the row spectra of the
@@ -794,10 +801,36 @@ struct Solve {
     // zero-padded filters (cuda_Pad_Dict + R2C, cbpdn.cu:277-289), computed
     // without materialising the padding.
     const bool rows_only = col_mode == COL_CONV && !full_dict;
+    const bool dict2d = !rows_only || o->record_itstat;
+    auto psum_rows = [&](const float* e, int E, const int* only) {
+      double2* R = (double2*)((unsigned char*)workspace + pl.off_lags);
+      const dim3 gr((g.Wf + 31) / 32, p->Kr, two_d ? 2 : 1), gp((g.Wf + 127) / 128, g.H);
+      if (only)
+        autocorr_kernel<true><<<gr, dim3(32, 8), 0, s>>>(e, R, g.M, p->Kr, E, g.Wf, g.Wp, only);
+      else
+        autocorr_kernel<false><<<gr, dim3(32, 8), 0, s>>>(e, R, g.M, p->Kr, E, g.Wf, g.Wp, only);
+      psum_lags_kernel<<<gp, 128, 0, s>>>(R, Psum, two_d ? Psum1 : nullptr,
+                                          two_d ? Psum0 : nullptr, g.H, g.Wf, g.Wp, p->Kr, only);
+      g_launches += 2;
+    };
+    auto dict_2d = [&](RowParams r, const int* only) -> int {
+      r.g.H = g.H;
+      r.held = only;
+      ColParams c = {};
+      c.g = g; c.g.B = 1; c.ph = pl.ph; c.twH = twH; c.twW = twW; c.F = Dh; c.held = only;
+      int e = launch_row<ROW_FWD_DICT>(pl, r, 1, s);
+      return e ? e : launch_col<COL_FWD>(pl, c, 1, s);
+    };
+    RowParams rd = {};
+    rd.g = g; rd.g.B = 1;
+    rd.pw = pl.pw; rd.twW = twW; rd.F = Dh; rd.D = p->D; rd.Kr = p->Kr; rd.Kc = p->Kc;
+    if (!spectra) {
+      if (Ep > 0 && dict2d && (st = dict_2d(rd, held))) return st;
+      if (two_d) psum_rows(Erows, Ep, held);
+      CU_TRY(cudaGetLastError());
+    }
     if (spectra) {
-      RowParams r = {};
-      r.g = g; r.g.B = 1;
-      r.pw = pl.pw; r.twW = twW; r.F = Dh; r.D = p->D; r.Kr = p->Kr; r.Kc = p->Kc;
+      RowParams r = rd;
       if (rows_only) r.g.H = p->Kr;  // Dh: (M, Kr, Wp)
       if ((st = launch_row<ROW_FWD_DICT>(pl, r, 1, s))) return st;
       // the row spectra of the filter rows, before the column transform
@@ -808,35 +841,22 @@ struct Solve {
         CU_TRY(cudaGetLastError());
         ++g_launches;
       }
-      const int ma = two_d ? 1 : 0;  // map 0 apart where its d differs
       if (rows_only) {
-        double2* R = (double2*)((unsigned char*)workspace + pl.off_lags);
-        const dim3 gr((g.Wf + 31) / 32, p->Kr), gp((g.Wf + 127) / 128, g.H);
-        for (int part = 0; part <= ma; ++part) {
-          const int lo = part ? 0 : ma, hi = part ? 1 : g.M;
-          autocorr_kernel<<<gr, dim3(32, 8), 0, s>>>(Dh, R, lo, hi, p->Kr, g.Wf, g.Wp);
-          psum_lags_kernel<<<gp, 128, 0, s>>>(R, part ? Psum0 : Psum, g.H, g.Wf, g.Wp, p->Kr);
-        }
+        psum_rows((const float*)Dh, p->Kr, nullptr);
         CU_TRY(cudaGetLastError());
-        g_launches += 2 + 2 * ma;
-        r.g.H = g.H;  // the functional's spectrum, in the place of the filter rows'
-        if (o->record_itstat && (st = launch_row<ROW_FWD_DICT>(pl, r, 1, s))) return st;
-      }
-      if (!rows_only || o->record_itstat) {
+        // the functional's spectrum, in the place of the filter rows'
+        if (dict2d && (st = dict_2d(r, nullptr))) return st;
+      } else {
         ColParams c = {};
         c.g = g; c.g.B = 1; c.ph = pl.ph; c.twH = twH; c.twW = twW; c.F = Dh;
         if ((st = launch_col<COL_FWD>(pl, c, 1, s))) return st;
-      }
-      if (!rows_only) {
         const size_t plane = (size_t)g.H * g.Wp;
-        psum_kernel<<<(unsigned)((plane + 255) / 256), 256, 0, s>>>(Dh + ma * plane, Psum,
-                                                                    g.M - ma, plane);
-        if (ma)
-          psum_kernel<<<(unsigned)((plane + 255) / 256), 256, 0, s>>>(Dh, Psum0, 1, plane);
+        psum_kernel<<<(unsigned)((plane + 255) / 256), 256, 0, s>>>(Dh, Psum, g.M, plane);
         CU_TRY(cudaGetLastError());
-        g_launches += 1 + ma;
+        ++g_launches;
       }
     }
+    const int made = (dict2d ? HELD_DICT : 0) | (two_d && rows_only ? HELD_SPLIT : 0);
     // Signal spectra (B images, one map each).
     if (spectra) {
       RowParams r = {};
@@ -853,10 +873,11 @@ struct Solve {
     if (o->warm_start) {
       // continue the state an earlier solve of this problem left in the
       // workspace: iterates, spectra of Y - U, rho, iteration count
-      warm_state_kernel<<<(g.B + 127) / 128, 128, 0, s>>>(sts, g.B, ndone);
+      warm_state_kernel<<<(g.B + 127) / 128, 128, 0, s>>>(sts, g.B, ndone, held, made, spectra);
     } else {
       if ((st = init_iterates())) return st;
-      init_state_kernel<<<(g.B + 127) / 128, 128, 0, s>>>(sts, p->rho0, g.B, ndone);
+      init_state_kernel<<<(g.B + 127) / 128, 128, 0, s>>>(sts, p->rho0, g.B, ndone, held, made,
+                                                          spectra);
     }
     xi_kernel<<<(g.B + 127) / 128, 128, 0, s>>>(xi, p->lmbda, g.B, o->rsdl_target,
                                                  o->std_residuals);
@@ -871,7 +892,7 @@ struct Solve {
     rp.bnd_c = o->no_bndry_cross && p->Kc > 1 ? g.W - (p->Kc - 1) : g.W;
     rp.partials = part; rp.st = sts; rp.vstate = vstate ? 1 : 0;
     cp.g = g; cp.ph = pl.ph; cp.twH = twH; cp.twW = twW; cp.F = F; cp.Dh = Dh; cp.Sh = Sh;
-    cp.grd = p->grd; cp.mu = p->mu; cp.wgrd = p->wgrd; cp.Psum = Psum; cp.st = sts;
+    cp.grd = p->grd; cp.mu = p->mu; cp.wgrd = p->wgrd; cp.Psum = two_d ? Psum1 : Psum; cp.st = sts;
     cp.E = Erows; cp.Kr = p->Kr; cp.Ep = Ep; cp.two = two_d ? 1 : 0; cp.Psum0 = Psum0;
     cp.twHd = (const double2*)((unsigned char*)workspace + pl.off_twHd);
     // The plain convolution solves write only their correction to the row
