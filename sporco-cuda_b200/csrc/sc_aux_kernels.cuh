@@ -162,6 +162,7 @@ __global__ void finalize_kernel(const double* __restrict__ partials, int nblk,
   // U as stored is the U of this iteration; the next row pass reads it scaled
   // by 1/rsf (U <- U / rsf, cbpdn.cu:543-549)
   S.uscale = 1.0 / rsf;
+  S.relay = 0;
   S.k = k;
   bool done = (r <= epri && s <= edua) || kc >= F.max_iter;
   if (!isfinite(r) || !isfinite(s)) {
@@ -181,7 +182,7 @@ __device__ __forceinline__ void note_held(int* held, int made, int over) {
 }
 
 __global__ void init_state_kernel(ImgState* st, const float* rho0, int B, int* ndone, int* held,
-                                  int made, int over) {
+                                  int made, int over, int paired) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b == 0) {
     *ndone = 0;
@@ -199,19 +200,24 @@ __global__ void init_state_kernel(ImgState* st, const float* rho0, int B, int* n
   s.done = 0;
   s.status = 0;
   s.k0 = 0;
+  s.paired = paired;
+  s.relay = 0;
   st[b] = s;
 }
 
 // A warm-started solve call continues the state of the previous one: rho,
 // the iterates and the iteration count carry over; the call's own cap counts
 // from the current count, and the finished flags start afresh.
-__global__ void warm_state_kernel(ImgState* st, int B, int* ndone, int* held, int made, int over) {
+__global__ void warm_state_kernel(ImgState* st, int B, int* ndone, int* held, int made, int over,
+                                  int paired) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b == 0) {
     *ndone = 0;
     note_held(held, made, over);
   }
   if (b >= B) return;
+  st[b].relay = st[b].paired != paired;
+  st[b].paired = paired;
   st[b].k0 = st[b].k;
   st[b].done = 0;
   st[b].status = 0;

@@ -79,6 +79,9 @@ struct ImgState {
   int done;      // 1: converged, iteration cap reached, or failed
   int status;    // sc_status of this image
   int k0;        // k at the start of the current solve call (its cap counts from here)
+  int paired;    // layout of F (RowParams::paired)
+  int relay;     // F is in the other layout still (a warm start with another column
+                 // pass): the fix-up at the start of the call writes it afresh
 };
 
 // What the workspace holds of the dictionary besides what every set-up leaves

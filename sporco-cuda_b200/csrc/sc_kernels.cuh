@@ -275,7 +275,7 @@ row_kernel(RowParams P) {
       rho = (float)st.rho;
       thr = (float)((double)P.lam[b] / st.rho);  // as the step's ROW_ITER had it
     } else {
-      if (st.rsf == 1.0) return;
+      if (st.rsf == 1.0 && !st.relay) return;
       rsf_c = (float)(1.0 - 1.0 / st.rsf);
       thr_prev = (float)((double)P.lam[b] / st.rho_prev);
       uscale = (float)st.uscale;
@@ -359,6 +359,7 @@ row_kernel(RowParams P) {
       // rows are staged one pair ahead (during the transform), F rows during
       // the next pair's packing.
       const bool vstate = P.vstate != 0;
+      const bool paired0 = paired != (P.st[b].relay != 0);  // layout that F has
       auto issue_U = [&](long p) {
         if (p < npairs) {
           const int n = ((2 * p + 1 < rows) ? 2 : 1) * W;
@@ -419,10 +420,10 @@ row_kernel(RowParams P) {
               spec_put(fa, k, A, paired);
               if (has1) spec_put(fa + Wp, k, Bv, paired);
             } else {
-              const float2 f0 = spec_get(fst, k, paired);
+              const float2 f0 = spec_get(fst, k, paired0);
               spec_put(fa, k, make_float2(f0.x + rsf_c * A.x, f0.y + rsf_c * A.y), paired);
               if (has1) {
-                const float2 f1 = spec_get(fst + Wp, k, paired);
+                const float2 f1 = spec_get(fst + Wp, k, paired0);
                 spec_put(fa + Wp, k, make_float2(f1.x + rsf_c * Bv.x, f1.y + rsf_c * Bv.y),
                          paired);
               }

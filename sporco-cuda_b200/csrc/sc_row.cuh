@@ -67,7 +67,7 @@ rowv_kernel(RowParams P) {
   if (st.done) return;
   float thr = 0.f, thr_prev;
   if constexpr (FIX) {
-    if (st.rsf == 1.0) return;
+    if (st.rsf == 1.0 && !st.relay) return;
     thr_prev = (float)((double)P.lam[b] / st.rho_prev);
   } else {
     thr = (float)((double)P.lam[b] / st.rho);
@@ -410,7 +410,7 @@ rowg_kernel(RowParams P) {
   if (st.done) return;
   float thr = 0.f, thr_prev;
   if constexpr (FIX) {
-    if (st.rsf == 1.0) return;
+    if (st.rsf == 1.0 && !st.relay) return;
     thr_prev = (float)((double)P.lam[b] / st.rho_prev);
   } else {
     thr = (float)((double)P.lam[b] / st.rho);

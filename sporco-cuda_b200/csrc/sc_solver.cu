@@ -856,6 +856,7 @@ struct Solve {
         ++g_launches;
       }
     }
+    const int paired = col_mode == COL_CONV && !full_dict;  // layout of F
     const int made = (dict2d ? HELD_DICT : 0) | (two_d && rows_only ? HELD_SPLIT : 0);
     // Signal spectra (B images, one map each).
     if (spectra) {
@@ -873,11 +874,12 @@ struct Solve {
     if (o->warm_start) {
       // continue the state an earlier solve of this problem left in the
       // workspace: iterates, spectra of Y - U, rho, iteration count
-      warm_state_kernel<<<(g.B + 127) / 128, 128, 0, s>>>(sts, g.B, ndone, held, made, spectra);
+      warm_state_kernel<<<(g.B + 127) / 128, 128, 0, s>>>(sts, g.B, ndone, held, made, spectra,
+                                                          paired);
     } else {
       if ((st = init_iterates())) return st;
       init_state_kernel<<<(g.B + 127) / 128, 128, 0, s>>>(sts, p->rho0, g.B, ndone, held, made,
-                                                          spectra);
+                                                          spectra, paired);
     }
     xi_kernel<<<(g.B + 127) / 128, 128, 0, s>>>(xi, p->lmbda, g.B, o->rsdl_target,
                                                  o->std_residuals);
@@ -904,7 +906,7 @@ struct Solve {
     // 100 maps, 25 iterations: 7e-7 -> 1.2e-6 relative; unmasked problems:
     // 3e-7 -> 2e-7 to 4e-7).
     rp.delta = col_mode == COL_CONV && conv_kind == CONV_DELTA;
-    rp.paired = col_mode == COL_CONV;
+    rp.paired = paired;
     fp.max_iter = o->max_iter;
     fp.auto_rho = o->auto_rho; fp.period = std::max(1, o->auto_rho_period);
     fp.auto_scaling = o->auto_scaling; fp.std_residuals = o->std_residuals;
@@ -919,7 +921,8 @@ struct Solve {
     if (o->warm_start) {
       // The last iteration of the earlier solve may have changed rho; its
       // fix-up of the row spectra (Y - U / rsf) did not run because that
-      // solve had finished.  Run it now (a no-op when rho did not change).
+      // solve had finished.  Run it now (a no-op when rho did not change and
+      // the column pass takes the layout that F has).
       if ((st = launch_row<ROW_FIXUP>(pl, rp, g.B, s))) return st;
     }
     if (tune && !o->warm_start && autotune_enabled() && o->max_iter > 0) {

@@ -72,3 +72,27 @@ def test_sums_of_another_weight_class(H, W, first, then):
     ref = _prepare(H, W, 6, then).run().cpu().numpy()
     _close(out[0], out[1])
     _close(out[0], ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,W", [(64, 64), (64, 33), (64, 48), (75, 33)])
+@pytest.mark.parametrize("warm", ["same", True])
+@pytest.mark.parametrize("given", [False, True])
+def test_column_pass_of_another_layout(H, W, warm, given):
+    """The same problem with another class named for its (equal) weights: the
+    other column pass wants the row spectra of Y - U in another layout.  Against
+    the continuation that keeps the class.  given: from given iterates (Y and U
+    kept apart).  Period 2 changes rho after the sixth iteration, not the fifth."""
+    for first in (5, 6):
+        out = []
+        for classes in ((2, 2, 2), (2, 0, 2)):
+            ds = _prepare(H, W, 6, ONE)
+            if given:
+                u0 = torch.full_like(ds.keep["Y"], 0.01)
+                ds.keep["Y"].fill_(0.02)
+                ds.prob.U0 = u0.data_ptr()
+            for n, c in enumerate(classes):
+                ds.prob.wgrd_uniform = c
+                Y = ds.run(warm=warm if n else False, iters=(first, 2, 3)[n])
+            out.append(Y.cpu().numpy())
+        _close(out[1], out[0])
