@@ -53,6 +53,8 @@ __host__ __device__ inline size_t rowg_slot_bytes(int W, int Wp) {
 // Column pass: radix-16 plans (16 elements per thread) for long columns,
 // radix-8 plans (8 per thread, twice the threads) for short ones.
 __host__ __device__ constexpr int col_radix(int H) { return H >= 512 ? 16 : 8; }
+// Shared memory that one CTA can have on sm_100a.
+#define SC_SMEM_MAX (227 * 1024)
 // Largest transform length this build supports along a row or a column.
 #define SC_MAX_N 4096
 
@@ -296,6 +298,14 @@ __host__ __device__ inline size_t conv_smem_bytes(int kind, int H, int L, int KR
   const size_t tl = conv_tile_entries(H, L, KR) * 8;
   return 3 * tl + (size_t)3 * KR * 64 + (kind == CONV_GRAD ? (size_t)4 * NT * 16 : 0) +
          (two ? tl : 0);
+}
+
+// Whether the convolution column pass of that kind fits (its default variant):
+// every length does but 2048 rows with map 0 apart, whose four tiles take 296 KB.
+inline bool conv_fits(int kind, int H, bool compiled, int Kr, bool two) {
+  const int n = compiled ? H : 0, L = conv_rows(n);
+  const int NT = compiled ? conv_threads(n, L) : conv_threads_any(H);
+  return conv_smem_bytes(kind, H, L, conv_pad_taps(Kr), NT, two) <= SC_SMEM_MAX;
 }
 
 __host__ __device__ inline size_t sc_align16(size_t x) { return (x + 15) & ~(size_t)15; }

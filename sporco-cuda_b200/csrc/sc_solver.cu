@@ -762,7 +762,8 @@ struct Solve {
     if (!p->grd && conv) {
       col_mode = COL_CONV;
       conv_kind = p->mask ? CONV_FULL : CONV_DELTA;
-    } else if (conv && p->wgrd_uniform >= 2 && p->mu >= 0.f && (!two || g.M >= 2)) {
+    } else if (conv && p->wgrd_uniform >= 2 && p->mu >= 0.f && (!two || g.M >= 2) &&
+               conv_fits(CONV_GRAD, g.H, spec_col(g.H), p->Kr, two)) {
       col_mode = COL_CONV;
       conv_kind = CONV_GRAD;
     } else if (p->grd) {
