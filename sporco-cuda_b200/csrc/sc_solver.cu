@@ -422,13 +422,15 @@ static int cluster_size(const void* fn, int NT, size_t smem, int M, long units, 
 }
 
 // Cluster sizes measured by the autotuner, per (device, kernel, image size,
-// maps); they replace the occupancy model's choice for that shape whatever
-// the number of images, so that a batch and a single solve of one size use
-// the same cluster size (the map reduction's summation order depends on it).
+// maps, and whether map 0 stands apart); they replace the occupancy model's
+// choice for that shape whatever the number of images, so that a batch and a
+// single solve of one size use the same cluster size (the map reduction's
+// summation order depends on it).
 struct TunedG {
   int dev;
   const void* fn;  // the kernel of the default radix (the key)
   int H, W, M;
+  int two;         // ColParams::two (a tile more of shared memory, two transforms more)
   int G;
   int rm;          // column-transform radix (8, or the default col_radix(H)); rows
                    // per thread of the convolution column pass
@@ -478,13 +480,13 @@ static int forced_split() {
   return G2 >= 1 && G2 <= 16 ? G2 : -1;
 }
 
-static bool tuned_size(const void* fn, const Geom& g, int* G, int* rm = nullptr,
+static bool tuned_size(const void* fn, const Geom& g, int two, int* G, int* rm = nullptr,
                        int* G2 = nullptr) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
   std::lock_guard<std::mutex> lock(g_cache_mu);
   for (const TunedG& e : g_tuned)
-    if (e.dev == dev && e.fn == fn && e.H == g.H && e.W == g.W && e.M == g.M) {
+    if (e.dev == dev && e.fn == fn && e.H == g.H && e.W == g.W && e.M == g.M && e.two == two) {
       *G = e.G;
       if (rm) *rm = e.rm;
       if (G2) *G2 = e.G2;
@@ -545,7 +547,7 @@ static int launch_clusters(const Plan& pl, ColParams cp, int B, cudaStream_t s, 
   int rm = force_rm, G2 = force_G2 > 0 ? force_G2 : 0;
   if (G <= 0) {
     int tG = 0, trm = 0, tG2 = 0;
-    if (tuned_size((const void*)v0.fn, cp.g, &tG, &trm, &tG2)) {
+    if (tuned_size((const void*)v0.fn, cp.g, cp.two, &tG, &trm, &tG2)) {
       G = tG;
       if (rm <= 0) rm = trm;
       if (force_G2 < 0) G2 = tG2;
@@ -1010,7 +1012,7 @@ struct Solve {
     const int rdef = iter_col_default();
     const void* fn = (const void*)iter_col_variant(rdef).fn;
     int G0 = 0;
-    if (forced_cluster(g.M) > 0 || tuned_size(fn, g, &G0)) return SC_OK;
+    if (forced_cluster(g.M) > 0 || tuned_size(fn, g, cp.two, &G0)) return SC_OK;
     int st;
     struct Cand { int rm, G; float ms; };
     std::vector<Cand> cand;
@@ -1085,10 +1087,11 @@ struct Solve {
       std::lock_guard<std::mutex> lock(g_cache_mu);
       bool known = false;
       for (const TunedG& e : g_tuned)
-        known = known || (e.dev == dev && e.fn == fn && e.H == g.H && e.W == g.W && e.M == g.M);
+        known = known || (e.dev == dev && e.fn == fn && e.H == g.H && e.W == g.W && e.M == g.M &&
+                          e.two == cp.two);
       if (!known)
         g_tuned.push_back(
-            {dev, fn, g.H, g.W, g.M, cand[bi].G, cand[bi].rm, best_G2});
+            {dev, fn, g.H, g.W, g.M, cp.two, cand[bi].G, cand[bi].rm, best_G2});
     }
     return init_iterates();
   }
@@ -1443,7 +1446,7 @@ static int unrolled_cluster(const Unrolled& u, int* G) {
   int st = prepare_fn((const void*)v.fn, true);
   if (st) return st;
   if ((*G = forced_cluster(u.pl.g.M)) > 0) return SC_OK;
-  if (tuned_size((const void*)v.fn, u.pl.g, G)) return SC_OK;
+  if (tuned_size((const void*)v.fn, u.pl.g, 0, G)) return SC_OK;
   return cluster_size((const void*)v.fn, v.NT, v.smem, u.pl.g.M,
                       (long)u.pl.col_ntiles * u.pl.g.B, v.Gmin, G);
 }
