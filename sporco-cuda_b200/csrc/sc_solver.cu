@@ -394,19 +394,18 @@ static int resident_clusters(const void* fn, int NT, size_t smem, int G, int* ou
 // autotuner's candidates).  Clusters lie within a GPC; with one CTA per SM a
 // size that divides the GPCs' SM counts badly leaves SMs idle, which sizes
 // other than the powers of two can avoid.
-static const int kClusterSizes[] = {8, 6, 4, 3, 2, 1};
+static const int kClusterSizes[] = {8, 6, 4, 3, 2};
 
 // CTAs per cluster of a clustered column launch over `units` column tiles
 // (tiles x images).  Candidates kClusterSizes (at most M); the estimated time
 // is (maps per CTA) x (rounds of resident clusters over the units), ties go
 // to the larger cluster.  Larger clusters split the maps more finely, smaller
 // ones pack the GPCs more tightly.
-static int cluster_size(const void* fn, int NT, size_t smem, int M, long units, int Gmin,
-                        int* G_out) {
+static int cluster_size(const void* fn, int NT, size_t smem, int M, long units, int* G_out) {
   int best = std::min(8, M);
   long best_cost = -1;
   for (int G : kClusterSizes) {
-    if (G > M || G < Gmin) continue;
+    if (G > M) continue;
     int nc = 0;
     int st = resident_clusters(fn, NT, smem, G, &nc);
     if (st) return st;
@@ -502,7 +501,6 @@ struct ColVariant {
   int NT = 0;
   size_t smem = 0;
   int g = 0;
-  int Gmin = 2;  // smallest cluster worth a trial
 };
 template <int MODE>
 static ColVariant col_variant(const Plan& pl, int rm) {
@@ -528,7 +526,6 @@ static ColVariant conv_variant(const Plan& pl, int kind, int Kr, int two, int L)
   v.fn = sc_colc_fn(kind, KR, n, L);
   v.NT = n > 0 ? conv_threads(n, L) : conv_threads_any(H);
   v.smem = conv_smem_bytes(kind, H, L, KR, v.NT, two);
-  v.Gmin = 1;
   return v;
 }
 
@@ -565,7 +562,7 @@ static int launch_clusters(const Plan& pl, ColParams cp, int B, cudaStream_t s, 
     if ((st = resident_clusters((const void*)v.fn, v.NT, v.smem, G, &n))) return st;
     if (n < 1) G = 0;
   }
-  if (G <= 0 && (st = cluster_size((const void*)v.fn, v.NT, v.smem, cp.g.M, units, v.Gmin, &G)))
+  if (G <= 0 && (st = cluster_size((const void*)v.fn, v.NT, v.smem, cp.g.M, units, &G)))
     return st;
   cp.gsz = v.g;
   // Tail split: the tiles past the last full round of one image's
@@ -1023,7 +1020,7 @@ struct Solve {
       if ((st = prepare_fn((const void*)v.fn, true))) return st;
       for (int G : kClusterSizes) {
         int n = 0;
-        if (G > g.M || G < v.Gmin) continue;
+        if (G > g.M) continue;
         if ((st = resident_clusters((const void*)v.fn, v.NT, v.smem, G, &n))) return st;
         if (n >= 1) cand.push_back({rm, G, 1e30f});
       }
@@ -1448,7 +1445,7 @@ static int unrolled_cluster(const Unrolled& u, int* G) {
   if ((*G = forced_cluster(u.pl.g.M)) > 0) return SC_OK;
   if (tuned_size((const void*)v.fn, u.pl.g, 0, G)) return SC_OK;
   return cluster_size((const void*)v.fn, v.NT, v.smem, u.pl.g.M,
-                      (long)u.pl.col_ntiles * u.pl.g.B, v.Gmin, G);
+                      (long)u.pl.col_ntiles * u.pl.g.B, G);
 }
 
 extern "C" size_t sc_unrolled_workspace_size(const sc_problem* p, const sc_options* o, int seg) {
