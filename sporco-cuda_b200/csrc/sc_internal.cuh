@@ -288,15 +288,15 @@ __host__ __device__ constexpr int conv_min_blocks(int kind, int n, int L, int KR
 }
 __host__ __device__ constexpr int conv_slots(int H, int L) { return L & 1 ? H : H + H / L; }
 // Shared memory of one CTA: three tiles of four columns (at least one map's
-// filter rows each), three maps' filter rows, the gradient term's carries and
-// map 0's tile.
+// filter rows each), three maps' filter rows, the gradient term's carries
+// and their weights, and map 0's tile.
 __host__ __device__ inline size_t conv_tile_entries(int H, int L, int KR) {
   const size_t a = (size_t)4 * conv_slots(H, L), b = (size_t)KR * 8;
   return a > b ? a : b;
 }
 __host__ __device__ inline size_t conv_smem_bytes(int kind, int H, int L, int KR, int NT, int two) {
   const size_t tl = conv_tile_entries(H, L, KR) * 8;
-  return 3 * tl + (size_t)3 * KR * 64 + (kind == CONV_GRAD ? (size_t)4 * NT * 16 : 0) +
+  return 3 * tl + (size_t)3 * KR * 64 + (kind == CONV_GRAD ? (size_t)NT * (4 * 16 + (L & 1 ? 16 : 8)) : 0) +
          (two ? tl : 0);
 }
 

@@ -36,7 +36,7 @@ def test_every_other_length_fits():
     def smem(H, L, KR, NT, two, grad=True):
         slots = H if L % 2 else H + H // L
         tile = max(4 * slots, KR * 8) * 8
-        return 3 * tile + 3 * KR * 64 + (4 * NT * 16 if grad else 0) + (tile if two else 0)
+        return 3 * tile + 3 * KR * 64 + (NT * (4 * 16 + (16 if L % 2 else 8)) if grad else 0) + (tile if two else 0)
 
     rows = {16: 4, 32: 4, 48: 6, 64: 4, 96: 4, 128: 4, 192: 8, 256: 8, 384: 8, 512: 8, 768: 8,
             1024: 8, 1536: 16, 2048: 16}
