@@ -210,7 +210,8 @@ rowv_kernel(RowParams P) {
             // to which the column pass has applied 1 / (H W)
             if constexpr (DL) x = fma2(pk2(v[m]), pk2(1.f, -1.f), sub2(yo, uo));
             else x = mul2(pk2(v[m]), pk2(P.invN, -P.invN));
-            const f32x2 vn = add2(fma2(a1, yo, mul2(a, x)), uo);
+            // (a x, the larger product, is the fused one; see iter_elem)
+            const f32x2 vn = add2(fma2(a, x, mul2(a1, yo)), uo);
             const float2 vv = up2(vn);
             const f32x2 y = soft2(vv, tc0, tc1);
             const f32x2 u = sub2(vn, y);
@@ -509,7 +510,8 @@ rowg_kernel(RowParams P) {
             z[k] = up2(sub2(yo, uo));
           } else {
             const f32x2 x = fma2(pk2(z[k]), xs, mul2(dl, sub2(yo, uo)));
-            const f32x2 vn = add2(fma2(a1, yo, mul2(a, x)), uo);
+            // (a x, the larger product, is the fused one; see iter_elem)
+            const f32x2 vn = add2(fma2(a, x, mul2(a1, yo)), uo);
             const float2 vv = up2(vn);
             const f32x2 y = soft2(vv, tc0, tc1);
             const f32x2 u = sub2(vn, y);
