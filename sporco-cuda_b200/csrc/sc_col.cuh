@@ -568,7 +568,7 @@ colc_kernel(ColParams P) {
                     "the CTA's threads cover whole columns");
 #pragma unroll 1
       for (int h = 0; h < T; h += CR)
-        fft_ct<NH, RMF, gF, T, 0, L, true>(tile + h + tid % CR, P.twH, tid / CR);
+        fft_ct<NH, RMF, gF, T, 0, L, 2>(tile + h + tid % CR, P.twH, tid / CR);
     } else {
       if (tile == A) fft_double(Z + (tid & 3), P.ph, T, P.twHd, tid >> 2, NT >> 2);
       else fft_forward<16>(tile + (tid & 3), P.ph, T, P.twH, tid >> 2, NT >> 2);

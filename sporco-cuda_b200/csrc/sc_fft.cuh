@@ -438,16 +438,25 @@ __device__ __forceinline__ void ptwiddle_r(float2* v, const float2* __restrict__
   }
 }
 
-// The butterfly and the twiddle products of a pass, scalar or packed (PK).  The
-// two fuse other products into their FMAs, so they differ in the last bit.
-template <int R, bool PK>
+// The same with every power from the table, to a rounding each.
+template <int R>
+__device__ __forceinline__ void ptwiddle_table(float2* v, const float2* __restrict__ tw, int i1) {
+#pragma unroll
+  for (int q = 1; q < R; ++q) v[q] = p_mul(v[q], __ldg(&tw[q * i1]));
+}
+
+// The butterfly and the twiddle products of a pass, scalar (PK = 0) or packed
+// (1; 2: the twiddles all from the table).  Scalar and packed ones fuse other
+// products into their FMAs, so they differ in the last bit.
+template <int R, int PK>
 __device__ __forceinline__ void dft_sel(float2* v) {
   if constexpr (PK) pdft_r<R>(v);
   else dft_r<R>(v);
 }
-template <int R, bool PK>
+template <int R, int PK>
 __device__ __forceinline__ void twiddle_sel(float2* v, const float2* __restrict__ tw, int i1) {
-  if constexpr (PK) ptwiddle_r<R>(v, tw, i1);
+  if constexpr (PK == 2) ptwiddle_table<R>(v, tw, i1);
+  else if constexpr (PK) ptwiddle_r<R>(v, tw, i1);
   else twiddle_r<R>(v, tw, i1);
 }
 
@@ -700,7 +709,7 @@ struct CtRun {
   }
 };
 
-template <int N, int RM, int R, int NS, int G, int ST, int BG = 0, int PAD = 0, bool PK = false>
+template <int N, int RM, int R, int NS, int G, int ST, int BG = 0, int PAD = 0, int PK = 0>
 __device__ __forceinline__ void ct_pass(float2* data, const float2* __restrict__ tw, int t) {
   constexpr int B = N / R;
   constexpr int NB = (B + G - 1) / G;
@@ -734,7 +743,7 @@ __device__ __forceinline__ void ct_pass(float2* data, const float2* __restrict__
   group_sync<BG>();
 }
 
-template <int N, int RM, int G, int ST, int BG = 0, int PAD = 0, bool PK = false, int P = 0>
+template <int N, int RM, int G, int ST, int BG = 0, int PAD = 0, int PK = 0, int P = 0>
 __device__ __forceinline__ void fft_ct(float2* data, const float2* __restrict__ tw, int t) {
   constexpr CtPlan pl = ct_plan(N, RM);
   if constexpr (P < pl.np) {
@@ -744,7 +753,7 @@ __device__ __forceinline__ void fft_ct(float2* data, const float2* __restrict__ 
 }
 
 // Passes [P, PEND) of a compile-time plan.
-template <int N, int RM, int G, int ST, int P, int PEND, int BG = 0, bool PK = false>
+template <int N, int RM, int G, int ST, int P, int PEND, int BG = 0, int PK = 0>
 __device__ __forceinline__ void fft_ct_passes(float2* data, const float2* __restrict__ tw, int t) {
   constexpr CtPlan pl = ct_plan(N, RM);
   if constexpr (P < PEND) {
@@ -769,7 +778,7 @@ __host__ __device__ constexpr bool ct_reg_edges(int n, int RM) {
 // First pass of a compile-time transform with its inputs in registers,
 // v[m] = element t + G m; results stored to shared memory.  Starts with a
 // barrier (PRE), so callers may still be reading the data array.
-template <int N, int RM, int ST, int BG = 0, bool PRE = true, bool PK = false>
+template <int N, int RM, int ST, int BG = 0, bool PRE = true, int PK = 0>
 __device__ __forceinline__ void ct_first_from_regs(float2* data, float2* v, int t) {
   constexpr CtPlan pl = ct_plan(N, RM);
   constexpr int R = pl.r[0];
@@ -785,7 +794,7 @@ __device__ __forceinline__ void ct_first_from_regs(float2* data, float2* v, int 
 
 // Last pass of a compile-time transform with its outputs left in registers,
 // v[m] = element t + G m.  Reads shared memory only.
-template <int N, int RM, int ST, bool PK = false>
+template <int N, int RM, int ST, int PK = 0>
 __device__ __forceinline__ void ct_last_to_regs(const float2* data,
                                                 const float2* __restrict__ tw, float2* v,
                                                 int t) {

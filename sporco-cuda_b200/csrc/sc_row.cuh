@@ -169,12 +169,12 @@ rowv_kernel(RowParams P) {
         if (m < EM / 2) v[m] = up2(fma2(pk2(A), pk2(1.f, -1.f), pk2(-B.y, -B.x)));
         else v[m] = up2(fma2(pk2(B.y, B.x), pk2(1.f, -1.f), pk2(A)));
       }
-      ct_first_from_regs<NW, RM, 1, BG, false, true>(z, v, t);
+      ct_first_from_regs<NW, RM, 1, BG, false, 1>(z, v, t);
       issue_V(p);  // the spectrum rows are consumed
-      fft_ct_passes<NW, RM, g, 1, 1, NP - 1, BG, true>(z, P.twW, t);
+      fft_ct_passes<NW, RM, g, 1, 1, NP - 1, BG, 1>(z, P.twW, t);
       cp_async_wait<0>();  // the state rows
       group_sync<BG>();
-      ct_last_to_regs<NW, RM, 1, true>(z, P.twW, v, t);
+      ct_last_to_regs<NW, RM, 1, 1>(z, P.twW, v, t);
     } else {
       cp_async_wait<0>();
       group_sync<BG>();
@@ -276,12 +276,12 @@ rowv_kernel(RowParams P) {
 #pragma unroll
       for (int m = 0; m < EM; ++m) v[m] = make_float2(0.f, 0.f);
     }
-    ct_first_from_regs<NW, RM, 1, BG, true, true>(z, v, t);
+    ct_first_from_regs<NW, RM, 1, BG, true, 1>(z, v, t);
     // the state rows are consumed: the next pair's rows land during this
     // pair's forward transform
     if constexpr (FIX) issue_V(p + pstride);
     else issue_F(p + pstride);
-    fft_ct_passes<NW, RM, g, 1, 1, NP, BG, true>(z, P.twW, t);
+    fft_ct_passes<NW, RM, g, 1, 1, NP, BG, 1>(z, P.twW, t);
     if (valid) {
       // A = (Z_k + conj Z_-k) / 2,  B = (Z_k - conj Z_-k) / 2i
       float2* fa = Fi + (size_t)r0 * Wp;
