@@ -38,10 +38,10 @@ RowFn sc_rowv_fn(int mode, int n, bool paired);
 // 128, 256; nullptr otherwise)
 RowFn sc_rowg_fn(int mode, int g);
 // sc_inst_row_iter.cu: ROW_ITER (other lengths), ROW_ITER_YU
-RowFn sc_row_fn_iter(int mode, int n);
+RowFn sc_row_fn_iter(int mode, int n, bool paired);
 // sc_inst_row_aux.cu: ROW_FIXUP, ROW_ADJ, ROW_FWD_REAL, ROW_INV_REAL,
 // ROW_FWD_DICT, ROW_FWD_YU
-RowFn sc_row_fn_aux(int mode, int n);
+RowFn sc_row_fn_aux(int mode, int n, bool paired);
 // sc_inst_colc*.cu: the convolution column pass, kind (ConvKind), kr padded
 // taps (8, 12, 16), at length n with L rows per thread (conv_rows(n) or
 // conv_rows_alt(n)); for a length without a compiled transform the variant for
@@ -65,11 +65,11 @@ __host__ __device__ constexpr bool col_has_r8(int mode) {
 }
 __host__ __device__ constexpr bool col_len_r8(int n) { return n == 512 || n == 768 || n == 1024; }
 
-// The table entry of MODE for length n.
+// The table entry of MODE for length n (paired: F in the paired layout).
 template <int MODE>
-inline RowFn row_fn(int n) {
-  if constexpr (MODE == ROW_ITER || MODE == ROW_ITER_YU) return sc_row_fn_iter(MODE, n);
-  else return sc_row_fn_aux(MODE, n);
+inline RowFn row_fn(int n, bool paired = false) {
+  if constexpr (MODE == ROW_ITER || MODE == ROW_ITER_YU) return sc_row_fn_iter(MODE, n, paired);
+  else return sc_row_fn_aux(MODE, n, paired);
 }
 template <int MODE>
 inline ColFn col_fn(int n) {

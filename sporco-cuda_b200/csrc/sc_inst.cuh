@@ -5,14 +5,14 @@
 #include "sc_dispatch.cuh"
 #include "sc_kernels.cuh"
 
-template <int MODE>
+template <int MODE, bool PL = false>
 RowFn row_table(int n) {
-#define SC_ROW_CASE(k) case k: return row_kernel<MODE, k>;
+#define SC_ROW_CASE(k) case k: return row_kernel<MODE, k, PL>;
   if constexpr (row_specialised(MODE)) {
     switch (n) { SC_SPEC_ROW(SC_ROW_CASE) default: break; }
   }
 #undef SC_ROW_CASE
-  return row_kernel<MODE, 0>;
+  return row_kernel<MODE, 0, PL>;
 }
 
 template <int MODE>

@@ -240,7 +240,8 @@ __device__ __forceinline__ float iter_elem(float x, float s0, float s1, const Ro
 // ============================================================== row pass ==
 // NW > 0: row length W known at compile time (specialised FFT plan);
 // NW == 0: any W (runtime FFT plan).
-template <int MODE, int NW>
+// PL: F in the paired layout (spec_re).
+template <int MODE, int NW, bool PL>
 __global__ void __launch_bounds__(SC_ROW_THREADS, row_min_blocks(NW))
 row_kernel(RowParams P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -284,7 +285,7 @@ row_kernel(RowParams P) {
     }
   }
 
-  const bool paired = P.paired != 0;  // layout of F (not the set-up modes')
+  constexpr bool paired = PL;  // layout of F (not the set-up modes')
   const long rows = (long)G.M * H;  // rows per image
   const long npairs = (rows + 1) / 2;
   const size_t img_real = (size_t)rows * W;

@@ -347,7 +347,7 @@ static int launch_row(const Plan& pl, RowParams rp, int B, cudaStream_t s, int n
   const bool rowg = !rowv && (MODE == ROW_ITER || MODE == ROW_FIXUP) && rp.vstate && !rp.plain &&
                     pl.rowg_smem_v > 0;
   if (rowg) fn = sc_rowg_fn(MODE, pl.rowg_g);
-  if (!rowv && !rowg) fn = row_fn<MODE>(rp.g.W);
+  if (!rowv && !rowg) fn = row_fn<MODE>(rp.g.W, rp.paired != 0);
   int st = prepare_fn((const void*)fn, false);
   if (st) return st;
   rp.gsz = hot ? pl.row_g : pl.rowg_g;
