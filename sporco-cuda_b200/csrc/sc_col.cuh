@@ -218,7 +218,7 @@ __device__ __forceinline__ void fft_double(double2* data, const FftPlan& P, int 
 // have to be those of one d: with d from 2 - 2 cos in 32 bits the error of a
 // column of 2048 rows was 3e-6 at mu w = 1e5 rho.)
 __device__ __forceinline__ float two_minus_2cos(float2 w) {
-  return w.x > 0.f ? 2.f * w.y * w.y / (1.f + w.x) : 2.f - 2.f * w.x;
+  return w.x > 0.f ? __fdividef(2.f * w.y * w.y, 1.f + w.x) : 2.f - 2.f * w.x;
 }
 
 template <int KIND, int KR, int NH, int L>
@@ -580,6 +580,14 @@ colc_kernel(ColParams P) {
   // conj(SC) / rho (DL: also times 1 / (H W), the row pass's normalisation of
   // its inverse transform)
   const float irho_s = DL ? (float)(1.0 / ((double)rho * H * G.W)) : irho;
+  // |G|^2 of this thread's columns but for the column frequency (e & 1 is tid & 1
+  // below)
+  float dc[2] = {0.f, 0.f};
+  if constexpr (GRD) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      dc[h] = two_minus_2cos(__ldg(&P.twW[min(c0 + 2 * cp + h, Wf - 1)]));
+  }
   fft(A);
   if (two) fft(W4);
   cp_async_wait<0>();
@@ -598,7 +606,7 @@ colc_kernel(ColParams P) {
           double2 q0 = make_double2(0.0, 0.0);
           double id = 1.0 / (double)rho, sd = 0.0;
           if (GRD)
-            id = 1.0 / ((double)Bw * (2.0 - 2.0 * P.twHd[kr].x + two_minus_2cos(P.twW[kc])) + rho);
+            id = 1.0 / ((double)Bw * (2.0 - 2.0 * P.twHd[kr].x + dc[h]) + rho);
           if (two) {
             const float4 w = reinterpret_cast<const float4*>(W4)[s4(e)];
             q0 = h ? make_double2(w.z, w.w) : make_double2(w.x, w.y);
@@ -638,8 +646,7 @@ colc_kernel(ColParams P) {
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int kc = min(c0 + c + h, Wf - 1);
-          const float id = 1.f / (Bw * (two_minus_2cos(__ldg(&P.twW[kc])) + ghr) + rho);
+          const float id = 1.f / (Bw * (dc[h] + ghr) + rho);
           const float sd = (h ? ps.y : ps.x) * id + (h ? p0.y : p0.x) * irho;
           const float rid = rho * id;
           const float g1 = 1.f / (1.f + sd);
@@ -772,37 +779,40 @@ colc_kernel(ColParams P) {
   int hops = 0;  // carries further away are below 2^-32 of their value
   if constexpr (GRD) {
     const int nb = (H + L - 1) / L;
-    float qv[2], gv[2], av[2], wv[NW][2], qm = 0.f;
+    float qv[2], gv[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int kc = min(c0 + 2 * cp + h, Wf - 1);
       const double Bd = Bw;
-      const double lo = (double)rho + Bd * two_minus_2cos(__ldg(&P.twW[kc]));  // A - 2 B
+      const double lo = (double)rho + Bd * dc[h];  // A - 2 B
       const double Ad = lo + 2.0 * Bd;
       qv[h] = fminf((float)(2.0 * Bd / (Ad + sqrt(lo * (lo + 4.0 * Bd)))), 0x1.fffffep-1f);
       const double q = qv[h];
       // H rho / (A - 2 B) (1 - q) / (1 + q): at d = A - 2 B the gain of both
       // recursions, 1 / (1 - q) + q / (1 - q), is 1 / d
-      gv[h] = (float)((double)hs * rho / lo * (1.0 - q) / (1.0 + q));
-      auto powq = [&](int n) {
-        double r = 1.0, p = q;
-        for (; n > 0; n >>= 1, p *= p)
-          if (n & 1) r *= p;
-        return r;
-      };
-      av[h] = (float)(1.0 / (1.0 - powq(H)));
-      // the weight of a block's end t blocks on, without the last, possibly
-      // short block among them and with it
-      wv[0][h] = (float)powq(L * t);
-      if constexpr (NW > 1) wv[1][h] = (float)powq(L * t - (nb * L - H));
-      qm = fmaxf(qm, qv[h]);
+      gv[h] = (float)((double)hs * rho * (1.0 - q) / (lo * (1.0 + q)));
     }
     q2 = pk2(qv[0], qv[1]);
     gain = pk2(gv[0], gv[1]);
-    around = pk2(av[0], av[1]);
-#pragma unroll
-    for (int i = 0; i < NW; ++i) Wt[i * NT + tid] = make_float2(wv[i][0], wv[i][1]);
+    const float qm = fmaxf(qv[0], qv[1]);
     hops = qm > 0.f ? (int)fminf((float)nb, 1.f + ceilf(-32.f / (L * log2f(qm)))) : 0;
+    auto powq = [&](int h, int n) {
+      double r = 1.0, p = qv[h];
+      for (; n > 0; n >>= 1, p *= p)
+        if (n & 1) r *= p;
+      return r;
+    };
+    // the weight of a block's end t blocks on, without the last, possibly short
+    // block among them and with it
+    if (t < hops) {
+      Wt[tid] = make_float2((float)powq(0, L * t), (float)powq(1, L * t));
+      if constexpr (NW > 1) {
+        const int n = L * t - (nb * L - H);
+        Wt[NT + tid] = make_float2((float)powq(0, n), (float)powq(1, n));
+      }
+    }
+    if (hops >= nb) {  // 1 / (1 - q^H)
+      around = pk2((float)(1.0 / (1.0 - powq(0, H))), (float)(1.0 / (1.0 - powq(1, H))));
+    }
   }
   int it = 0;
   for (int m = m0; m < m1; ++m, ++it) {
