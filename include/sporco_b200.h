@@ -254,7 +254,7 @@ unsigned long long sc_launch_count(void);
  *     every seg iterations in the workspace (seg: 1..K; ceil(sqrt(K)) balances memory
  *     against the one recomputation of each segment in the backward pass;
  *     seg = K with filters of at most 16 rows and compiled column lengths
- *     below 512 keeps the trace of every step instead, so that the backward
+ *     below 512 but 96 keeps the trace of every step instead, so that the backward
  *     recomputes nothing, in a workspace of about K (R + C) bytes).
  *   sc_unrolled_backward, after a forward call with the same problem,
  *     options, seg and workspace, takes gY = dLoss/dY_K (B, M, H, W) and
