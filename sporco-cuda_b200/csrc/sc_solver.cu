@@ -147,7 +147,7 @@ struct Plan {
   int colg_g, colg_NT;
   size_t colg_smem, colt_smem;
   int max_iter;
-  bool pdl;  // programmatic launches
+  bool pdl, pdl_col;  // programmatic launches; of the clustered column passes
   size_t off_U, off_F, off_Dh, off_Sh, off_Ps, off_Ps0, off_Ps1, off_E, off_twW, off_twH, off_twHd, off_lags, off_part, off_st,
       off_held, off_it, off_xi, off_ndone, off_objspec, off_objpart, total;
 };
@@ -179,7 +179,7 @@ static int num_sms() {
   return n;
 }
 
-static bool pdl_enabled(const Geom& g, bool conv);
+static bool pdl_enabled(const Geom& g);
 static int plan_geometry(int B, int M, int H, int W, Plan* pl) {
   if (B < 1 || M < 1 || H < 1 || W < 1)
     return set_status(SC_ERR_INVALID, "sizes must be positive (B=%d M=%d H=%d W=%d)", B, M, H, W);
@@ -192,7 +192,7 @@ static int plan_geometry(int B, int M, int H, int W, Plan* pl) {
   g.Wp = (g.Wf + 3) & ~3;
   if (make_fft_plan(W, &pl->pw) || make_fft_plan(W, &pl->pwo, true) || make_fft_plan(H, &pl->ph))
     return set_status(SC_ERR_UNSUPPORTED, "cannot factor %d or %d", W, H);
-  pl->pdl = pdl_enabled(g, false);
+  pl->pdl = pl->pdl_col = pdl_enabled(g);
   const bool srow = spec_row(W), scol = spec_col(H);
   const int zlen = srow ? ct_len(W, row_radix(W), 1) : W;
   pl->row_g = srow ? ct_threads(W, row_radix(W)) : group_size(W);
@@ -234,7 +234,7 @@ static int plan_problem(const sc_problem* p, const sc_options* o, Plan* pl) {
   if (p->Kr < 1 || p->Kc < 1 || p->Kr > p->H || p->Kc > p->W)
     return set_status(SC_ERR_INVALID, "filter size %dx%d invalid for image %dx%d", p->Kr, p->Kc,
                       p->H, p->W);
-  pl->pdl = pdl_enabled(pl->g, p->Kr <= 16);
+  pl->pdl_col = pl->pdl && !o->auto_rho;  // (no fix-up before it)
   if (o->max_iter < 0) return set_status(SC_ERR_INVALID, "max_iter < 0");
   pl->max_iter = o->max_iter;
   const Geom& g = pl->g;
@@ -302,35 +302,27 @@ static int prepare_fn(const void* fn, bool cluster) {
 // length has one; the setup modes always use the runtime plan.
 // Programmatic dependent launch of the solver's kernels (each waits for the
 // kernel before it at its start): the next kernel's CTAs are scheduled while
-// the previous one drains, which hides the gaps between short kernels, but
-// they hold SMs that the previous kernel's last clusters could use.  Measured on
-// whole solves of 40 iterations at 7 column lengths (100 and 317 without a
-// compiled transform) by 5 row lengths from 64 to 1024, 8 to 128 maps, 8, 12, 16
-// and 18 taps, plain, masked, with the gradient term and both; time with them over
-// time without:
-//   up to 0.2 million coefficients                   0.66 to 1.06 (64 x 64, 32
-//                                                    maps 0.70 to 0.79)
-//   to 0.3 million, compiled column lengths          0.74 to 1.10, mean 0.87
-//   to 5 million, compiled column lengths,
-//     transform column solves                        0.78 to 1.04
-//     convolution pass, at most 64 or at least 1024
-//     rows, or rows of 512 and more                  0.76 to 1.07, mean 0.9
-//     convolution pass, other sizes                  0.80 to 1.35, mean 1.03
-//   column lengths without a compiled transform      0.85 to 1.62, mean 1.05
-//   beyond 5 million                                 0.93 to 1.37, mean 1.03
-// Only with rowv_kernel's row lengths (475 x 315, 8 maps 6.69 -> 7.28 ms, 100 x 75,
-// 32 maps 2.99 -> 3.13).  SPORCO_B200_PDL=1 / 0: on / off for every problem.
-// conv: the filters are short enough for the convolution pass.
-static bool pdl_enabled(const Geom& g, bool conv) {
+// the previous one drains, which hides the gaps between short kernels.  For
+// problems of up to 12 million coefficients with rowv_kernel's row lengths (475 x
+// 315, 8 maps 6.69 -> 7.28 ms, 100 x 75, 32 maps 2.99 -> 3.13 with it).  Not for the
+// clustered column pass where the fix-up runs before it (adaptive rho): its CTAs
+// would take the shared memory from an active fix-up's.  Solves of 40 iterations at
+// 5 column lengths (317 without a compiled transform) by row lengths of 64, 128,
+// 256 and 512, 8 to 128 maps, 8, 12, 16 and 18 taps, plain, masked and with the
+// gradient term; time with programmatic launches over time without:
+//   adaptive rho, the column pass launched plainly    0.73 to 1.02, mean 0.91
+//   adaptive rho, the column pass as well             0.66 to 1.62, mean 0.99
+//   rho fixed, the column pass as well                0.70 to 1.07, mean 0.91
+// (64 x 64, 32 maps 0.76 to 0.85; 200 x 128, 24 maps of 5 x 5, adaptive rho, 2.37 ms
+// plainly, 2.98 with the column pass launched so.)  SPORCO_B200_PDL=1 / 0: on / off
+// for every problem.
+static bool pdl_enabled(const Geom& g) {
   static const int set = [] {
     const char* e = getenv("SPORCO_B200_PDL");
     return e && e[0] == '1' ? 1 : e && e[0] == '0' ? 0 : -1;
   }();
-  if (set >= 0) return set > 0;
-  if (!spec_row(g.W) || !rowv_len(g.W)) return false;
-  const double n = (double)g.B * g.M * g.H * g.W;
-  if (n <= (spec_col(g.H) ? 0.3e6 : 0.2e6)) return true;
-  return n <= 5e6 && spec_col(g.H) && (!conv || g.H <= 64 || g.H >= 1024 || g.W >= 512);
+  return set >= 0 ? set > 0
+                  : spec_row(g.W) && rowv_len(g.W) && (double)g.B * g.M * g.H * g.W <= 12e6;
 }
 static void set_pdl(cudaLaunchAttribute* a) {
   a->id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -614,7 +606,7 @@ static int launch_clusters(const Plan& pl, ColParams cp, int B, cudaStream_t s, 
     attr[0].val.clusterDim.z = 1;
     set_pdl(&attr[1]);
     cfg.attrs = attr;
-    cfg.numAttrs = pl.pdl ? 2 : 1;
+    cfg.numAttrs = pl.pdl_col ? 2 : 1;
     CU_TRY(cudaLaunchKernelEx(&cfg, v.fn, cp));
     ++g_launches;
   }
