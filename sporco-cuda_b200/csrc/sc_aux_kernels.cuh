@@ -69,7 +69,7 @@ __global__ void autocorr_kernel(const float* __restrict__ e, double2* __restrict
 // two slices of R also Psum1 of the maps [1, M) and Psum0 of map 0.
 // (Instead of the zero-padded filters' 2-D spectra and a sum over the maps:
 // 2048 x 2048, 256 filters of 16 x 16 11.4 -> 0.3 ms of a solve's set-up, 256 x
-// 256, 64 of 11 x 11 80 -> 20 us.)
+// 256, 64 of 11 x 11 80 -> 28 us.)
 __global__ void psum_lags_kernel(const double2* __restrict__ R, float* __restrict__ Psum,
                                  float* __restrict__ Psum1, float* __restrict__ Psum0, int H,
                                  int Wf, int Wp, int Kr, const int* held) {

@@ -28,13 +28,14 @@
 //             circular, instead of two transforms per map.
 //
 // Measured per launch (before -> now): CONV_DELTA 2048 x 2048, 256 maps, 16
-// taps 3.41 -> 2.94 ms; 256 x 256, 64 maps, 8 taps 26.0 -> 17.7 us; 64 x 64, 32
-// maps 13.5 -> 7.5 us.  CONV_FULL 512 x 512, 101 maps, 12 taps 115 -> 99 us.
-// CONV_GRAD 512 x 512, 100 maps 209 (two transforms per map) -> 110 us; with the
-// impulse map 384 x 512, 65 maps, 8 taps 165 (COL_SOLVE_W) -> 68 us.  Without a
-// compiled column length 3 x 320 x 480, 36 maps, 8 taps 266 (COL_SOLVE_P) -> 91
-// us.  Bound by the window loads' and the FMAs' latencies at 8 to 12 warps per
-// SM (registers; FMA pipe 40 to 60 % busy), DRAM a third busy.
+// taps 3.41 -> 2.99 ms (at 1965 MHz; 3.2 ms under the power cap of a long solve);
+// 256 x 256, 64 maps, 8 taps 26.0 -> 17.7 us; 64 x 64, 32 maps 13.5 -> 7.5 us.
+// CONV_FULL 512 x 512, 101 maps, 12 taps 115 -> 99 us.  CONV_GRAD 512 x 512, 100
+// maps 209 (two transforms per map) -> 110 us; with the impulse map 384 x 512, 65
+// maps, 8 taps 165 (COL_SOLVE_W) -> 68 us.  Without a compiled column length 3 x
+// 320 x 480, 36 maps, 8 taps 266 (COL_SOLVE_P) -> 91 us.  Bound by the window
+// loads' and the FMAs' latencies at 8 to 12 warps per SM (registers; FMA pipe 40
+// to 60 % busy), DRAM a third busy.
 //
 // Each thread owns L consecutive rows of two adjacent columns and does both in
 // packed FP32 instructions, in Gauss's three-multiply form (e = c + i d,

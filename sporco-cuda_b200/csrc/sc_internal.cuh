@@ -271,7 +271,7 @@ __host__ __device__ constexpr int conv_radix(int n) { return n >= 192 ? 16 : 8; 
 __host__ __device__ constexpr int conv_sweep(int KR, int L) { return KR == 16 ? 8 : KR; }
 // Complex products in Gauss's form (three packed FMAs) or plainly (four); both
 // measured: 256 x 256, 8 taps 17.7 / 18.5 us, 512 x 512, 12 taps 99 / 108 us,
-// 2048 x 2048, 16 taps 2.94 / 3.25 ms, 64 x 64, 8 taps 8.0 / 7.5 us, 320 rows
+// 2048 x 2048, 16 taps 2.95 / 3.25 ms, 64 x 64, 8 taps 8.0 / 7.5 us, 320 rows
 // (not compiled) 78.3 / 78.6 us.
 __host__ __device__ constexpr bool conv_gauss(int n) { return n > 128; }
 // Resident CTAs per SM the kernel is compiled for: as many as its registers
@@ -296,8 +296,8 @@ __host__ __device__ inline size_t conv_tile_entries(int H, int L, int KR) {
 }
 __host__ __device__ inline size_t conv_smem_bytes(int kind, int H, int L, int KR, int NT, int two) {
   const size_t tl = conv_tile_entries(H, L, KR) * 8;
-  return 3 * tl + (size_t)3 * KR * 64 + (kind == CONV_GRAD ? (size_t)NT * (4 * 16 + (L & 1 ? 16 : 8)) : 0) +
-         (two ? tl : 0);
+  return 3 * tl + (size_t)3 * KR * 64 +
+         (kind == CONV_GRAD ? (size_t)NT * (4 * 16 + (L & 1 ? 16 : 8)) : 0) + (two ? tl : 0);
 }
 
 // Whether the convolution column pass of that kind fits (its default variant):

@@ -24,8 +24,9 @@
 // Measured per launch against row_kernel (256-thread CTAs in lock step, a
 // staging buffer each for spectrum and state rows), ITER / FIXUP active:
 // 2048 x 2048, 256 maps 4.99 -> 3.93 ms / 2.37 -> 1.9 ms (17.2 / 8.6 GB: 4.4
-// TB/s); 512 x 512, 100 maps 130 -> 101 us; 256 x 256, 64 maps 26 -> 18 us;
-// 64 x 64, 32 maps 7.2 -> 4.7 us.
+// TB/s; at 1965 MHz; 4.2 to 4.4 ms within a 100-iteration solve, where the power
+// cap holds the clock at 1820 to 1890 MHz); 512 x 512, 100 maps 130 -> 101 us;
+// 256 x 256, 64 maps 26 -> 18 us; 64 x 64, 32 maps 7.2 -> 4.7 us.
 #pragma once
 
 #include "sc_kernels.cuh"
